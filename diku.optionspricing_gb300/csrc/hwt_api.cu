@@ -262,22 +262,25 @@ int check_config(hwt_ctx *c, const hwt_config &cfg)
 
 
 // How the GPU reaches a caller's host pointer: `dev` its address in a kernel (null if it
-// has none), `pinned` page-locked memory.  On a coherent host (c->host_coherent) kernels
-// read pageable memory at its own address.
+// has none, or is not aligned to its elements' size, as arrays inside a byte buffer may not
+// be: a kernel's load from there would fault, so these take the copies), `pinned`
+// page-locked memory.  On a coherent host (c->host_coherent) kernels read pageable memory
+// at its own address.
 struct HostView {
     const void *dev;
     bool pinned;
 };
 
-HostView host_view(const hwt_ctx *c, const void *p)
+HostView host_view(const hwt_ctx *c, const void *p, size_t size)
 {
+    const bool aligned = reinterpret_cast<uintptr_t>(p) % size == 0;
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
         return {nullptr, false};
     }
-    if (at.type == cudaMemoryTypeHost) return {at.devicePointer, true};
-    return {at.type == cudaMemoryTypeUnregistered && c->host_coherent ? p : nullptr, false};
+    if (at.type == cudaMemoryTypeHost) return {aligned ? at.devicePointer : nullptr, true};
+    return {aligned && at.type == cudaMemoryTypeUnregistered && c->host_coherent ? p : nullptr, false};
 }
 
 // Option arrays in host memory (src) into the packed device arrays (dst): one pass by a
@@ -614,9 +617,9 @@ int hwt_price_ex(hwt_ctx *c, const hwt_options *o, const hwt_yield *y, const hwt
     const int grid = cfg.mode == HWT_PLAIN_FP64 ? 0 : pricing_blocks_per_sm(cfg.mode) * c->sms;
     int launches = 0, launches_before = 0, graph_used = 0;
     // the option arrays (in the order of the SoA record) and the output
-    const HostView v[9] = {host_view(c, o->strike), host_view(c, o->bond_maturity), host_view(c, o->option_maturity),
-                           host_view(c, o->term_unit), host_view(c, o->term_steps), host_view(c, o->a),
-                           host_view(c, o->sigma), host_view(c, o->type), host_view(c, out)};
+    const HostView v[9] = {host_view(c, o->strike, 8), host_view(c, o->bond_maturity, 8), host_view(c, o->option_maturity, 8),
+                           host_view(c, o->term_unit, 2), host_view(c, o->term_steps, 2), host_view(c, o->a, 8),
+                           host_view(c, o->sigma, 8), host_view(c, o->type, 1), host_view(c, out, 8)};
     bool reachable = true, pinned = true;
     for (int i = 0; i < 8; ++i) {
         reachable = reachable && v[i].dev;
@@ -633,7 +636,7 @@ int hwt_price_ex(hwt_ctx *c, const hwt_options *o, const hwt_yield *y, const hwt
     host.a = (const double *)v[5].dev;
     host.sigma = (const double *)v[6].dev;
     host.type = (const int8_t *)v[7].dev;
-    if (c->host_coherent && pinned && out_pinned) {
+    if (c->host_coherent && pinned && reachable && out_pinned) {
         // Pinned caller arrays on a host that the GPU reaches coherently
         // (NVLink-C2C): the sizing kernel reads the option fields where they are
         // (one pass over 45 bytes per option, no copies in); the prices go to
