@@ -43,3 +43,16 @@ def test_small_prices_keep_their_digits(pkg, pricer, batch, mode_name):
     rel = np.abs(got - ref)[some] / ref[some]
     assert np.max(rel) <= BOUND[mode_name], (np.max(rel), ref[some][np.argmax(rel)])
     assert np.max(got[~some], initial=0.0) <= 2 * SMALLEST[mode_name]
+
+
+@pytest.mark.parametrize("mode_name", ["BATCHED_FP32", "BATCHED_MIXED"])
+def test_cut_float_trees_keep_small_prices(pkg, pricer, batch, mode_name):
+    """The cut leaves out paths of weight exp(-34) of the price, not of the bond: cut and
+    uncut prices agree to float rounding at every size that float rows hold."""
+    opts, y, ref = batch
+    mode = getattr(pkg, mode_name)
+    uncut = pricer.price(opts, y, mode, big_threshold=1024)
+    cut = pricer.price(opts, y, mode)
+    some = uncut > 1e-25
+    assert some.sum() > 800
+    assert np.max(np.abs(cut - uncut)[some] / uncut[some]) <= 2.0 ** -20
