@@ -166,15 +166,9 @@ struct PolyTable {
     int32_t n_max;
 };
 
-// A number as the path's scalars hold it: a double, or a double-float pair.
-union PolyScal {
-    double d;
-    float2 f;
-};
-
 // One tree of the polynomial path (in the tree's Tree slot).
 struct PolyTree {
-    PolyScal M, drdt, X, fwd, pm;  // exp(-a dt) - 1; dr dt; strike; 100 P_n / P_m; P_m
+    double M, drdt, X, fwd, pm;    // exp(-a dt) - 1; dr dt; strike; 100 P_n / P_m; P_m
     int32_t idx;
     int32_t row_f, row_b;          // coefficient rows of the two powers
     int16_t df, db, J;
