@@ -73,7 +73,8 @@ struct hwt_ctx {
     double *d_yrate = nullptr;
     float *d_yrate_f = nullptr;
     int32_t *d_yday = nullptr;
-    void *d_table = nullptr;     // coefficient table of the polynomial path
+    void *d_table = nullptr;     // coefficient table of the polynomial path, and the view of it
+    PolyTable table = {};
     int64_t device_bytes = 0;
 
     // pinned host staging
@@ -387,7 +388,7 @@ int run_batch(hwt_ctx *c, const DevOptions &dopt, double *dev_out, const RunConf
         }
     }
     p.s.cta_busy = c->d_busy;
-    p.tab = poly_table_view(c->d_table, kPolyMaxN);
+    p.tab = c->table;
     poly_params(p, cfg.mode, cfg.given_threshold, cfg.given_k_mask, c->sms, grid);
 
     const bool timing = stats != nullptr;
@@ -537,8 +538,9 @@ hwt_ctx *hwt_create(int device, const char *tune_cache)
     ok = ok && cudaHostAlloc((void **)&c->h_yday, 4 * kMaxYield, cudaHostAllocDefault) == cudaSuccess;
     const size_t table_bytes = poly_table_bytes(kPolyMaxN);
     ok = ok && cudaMalloc(&c->d_table, table_bytes) == cudaSuccess &&
-         cudaMemsetAsync(c->d_table, 0, table_bytes, c->stream) == cudaSuccess &&
-         launch_poly_table(c->d_table, kPolyMaxN, c->stream) == cudaSuccess;
+         cudaMemsetAsync(c->d_table, 0, table_bytes, c->stream) == cudaSuccess;
+    c->table = poly_table_view(c->d_table, kPolyMaxN);
+    ok = ok && launch_poly_table(c->table, c->stream) == cudaSuccess;
     for (int m = 0; m < kNumModes; ++m) {
         hwt_config &t = c->tuned[m];
         memset(&t, 0, sizeof(t));

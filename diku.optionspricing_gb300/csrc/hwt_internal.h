@@ -113,6 +113,7 @@ constexpr int kPolyThreadsFP64 = 384;
 constexpr int kPolyThreadsDF64 = 512;
 constexpr int kPolyMaxJ = 128 * 8 / 2 - 1;
 constexpr int kPolyMaxN = 4096;         // tallest tree with a coefficient row
+constexpr int kPolyNoAllocN = 1024;     // the allocation-free entry point's table
 constexpr int kPolyBuckets = 64;
 constexpr int kPolySplits = 8;
 constexpr int kPolyClasses = kNumPolyK * kPolyL;
@@ -162,6 +163,7 @@ struct PolyTable {
     const long long *fixed;  // times 2^kFixedTable
     const float *hi, *lo;
     const int32_t *off;    // [n_max + 2]
+    int32_t *filled;       // [n_max + 1]: rows that are filled (zero at first)
     const uint16_t *deg;   // [(POLY_LEVELS + 1) * (n_max + 1)]
     int32_t n_max;
 };
@@ -240,11 +242,11 @@ int pricing_blocks_per_sm(int mode);
 // Polynomial path (hwt_poly.cu): its fields of a run, its kernel, and the table.
 void poly_params(EngineParams &p, int mode, int explicit_threshold, int explicit_k_mask, int sms, int grid);
 cudaError_t launch_poly(const EngineParams &p, int mode, int grid, cudaStream_t stream);
-// Coefficient table for heights up to n_max: bytes of its one buffer, and the kernel
-// that fills it (once; a filled buffer is left alone) and the view of it.
+// Coefficient table for heights up to n_max (kPolyMaxN or kPolyNoAllocN): bytes of its one
+// buffer, zero at first, the view of it, and the kernel that fills it.
 size_t poly_table_bytes(int n_max);
-cudaError_t launch_poly_table(void *buffer, int n_max, cudaStream_t stream);
 PolyTable poly_table_view(void *buffer, int n_max);
+cudaError_t launch_poly_table(const PolyTable &t, cudaStream_t stream);
 cudaError_t launch_plain(const EngineParams &p, int max_width, int max_height, cudaStream_t stream);
 size_t plain_smem_bytes(int max_width, int max_height);
 int sizing_launches();

@@ -29,6 +29,7 @@
 
 #include "../../include/hwtree.h"
 #include "hwt_internal.h"
+#include "hwt_poly.cuh"
 
 using namespace hwt;
 
@@ -55,10 +56,9 @@ constexpr size_t kScratchBytes = up(kOffCurveBad + 4);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
-// Coefficient table of the polynomial path for heights up to kNoAllocMaxN (taller trees
-// take the general path): filled by the first call in a context (the array is zero when
-// the context loads it, and with it the table's own mark), kept after that.
-constexpr int kNoAllocMaxN = 1024;
+// Coefficient table of the polynomial path for heights up to kPolyNoAllocN (taller trees
+// take the general path): filled by the first double-mode call in a context (the array is
+// zero when the context loads it, and with it the rows' marks), kept after that.
 constexpr size_t isqrt_up(size_t v)
 {
     size_t r = 0;
@@ -72,18 +72,22 @@ constexpr size_t table_bound(int n_max)  // poly_table_bytes, from above
         const size_t d = 10 * isqrt_up(N) + 8;
         entries += (d < (size_t)N ? d : (size_t)N) + 1;
     }
-    return up(24 * entries + 12 * ((size_t)n_max + 3) + 64);
+    return up(24 * entries + 16 * ((size_t)n_max + 3) + 64);
 }
-static __device__ __align__(256) unsigned char g_noalloc_table[table_bound(kNoAllocMaxN)];
+static __device__ __align__(256) unsigned char g_noalloc_table[table_bound(kPolyNoAllocN)];
 
-// Float copy of the curve; *bad is raised for a rate that is not finite.
-__global__ void curve_to_float(const double *rate, int n, float *rate_f, int *bad)
+// Float copy of the curve (*bad is raised for a rate that is not finite), and in the double
+// mode the table's rows that are not filled yet.
+constexpr int kSetupThreads = 64;
+__global__ void setup_kernel(const double *rate, int n, float *rate_f, int *bad, PolyTable table, int fill)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double r = rate[i];
-    if (!isfinite(r)) atomicExch(bad, 1);
-    rate_f[i] = (float)r;
+    if (i < n) {
+        const double r = rate[i];
+        if (!isfinite(r)) atomicExch(bad, 1);
+        rate_f[i] = (float)r;
+    }
+    if (fill) poly_fill_row(table, i);
 }
 
 int fail_cuda(cudaError_t e)
@@ -117,7 +121,7 @@ extern "C" int hwt_price_device_noalloc(const hwt_options *dev_opts, const hwt_y
     unsigned char *base = (unsigned char *)scratch;
     void *table = nullptr;
     if ((e = cudaGetSymbolAddress(&table, g_noalloc_table)) != cudaSuccess) return fail_cuda(e);
-    if (poly_table_bytes(kNoAllocMaxN) > sizeof(g_noalloc_table)) return HWT_EUNSUPPORTED;
+    if (poly_table_bytes(kPolyNoAllocN) > sizeof(g_noalloc_table)) return HWT_EUNSUPPORTED;
 
     EngineParams p;
     memset(&p, 0, sizeof(p));
@@ -160,15 +164,15 @@ extern "C" int hwt_price_device_noalloc(const hwt_options *dev_opts, const hwt_y
     const int per = pricing_blocks_per_sm(mode);
     if (per < 1) return HWT_EUNSUPPORTED;
 
-    p.tab = poly_table_view(table, kNoAllocMaxN);
+    p.tab = poly_table_view(table, kPolyNoAllocN);
     poly_params(p, mode, 0, 0, sms, per * sms);
 
     int *curve_bad = (int *)(base + kOffCurveBad);
     if ((e = cudaMemsetAsync(curve_bad, 0, sizeof(int), st)) != cudaSuccess) return fail_cuda(e);
-    curve_to_float<<<(dev_yield->n + 255) / 256, 256, 0, st>>>(dev_yield->rate, dev_yield->n, (float *)(base + kOffRateF),
-                                                               curve_bad);
+    const int rows = p.poly ? kPolyNoAllocN + 1 : 0, items = dev_yield->n > rows ? dev_yield->n : rows;
+    setup_kernel<<<(items + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0, st>>>(
+        dev_yield->rate, dev_yield->n, (float *)(base + kOffRateF), curve_bad, p.tab, p.poly);
     if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(e);
-    if (p.poly && (e = launch_poly_table(table, kNoAllocMaxN, st)) != cudaSuccess) return fail_cuda(e);
     // launch_sizing clears the histogram, fill counters and run status itself
     if ((e = launch_sizing(p, st)) != cudaSuccess) return fail_cuda(e);
     if ((e = launch_pricing(p, mode, per * sms, st)) != cudaSuccess) return fail_cuda(e);
