@@ -227,7 +227,8 @@ bool valid_sort(int s)
 bool wide_rows(int mode) { return mode == HWT_BATCHED_FP64 || mode == HWT_BATCHED_DF64; }
 
 // A call's configuration: the caller's fields over the context's, and which layout
-// limits the caller gave (0: none).
+// limits the caller gave (0: none).  A whole record, with group size, threshold and K set (as
+// hwt_get_config and hwt_autotune return it), is a configuration and no limit.
 struct RunConfig : hwt_config {
     int given_threshold, given_k_mask;
 };
@@ -237,8 +238,9 @@ RunConfig resolve(const hwt_ctx *c, const hwt_config *cfg, int mode)
     RunConfig r;
     static_cast<hwt_config &>(r) = c->tuned[(mode >= 0 && mode < kNumModes) ? mode : 0];
     r.mode = mode;
-    r.given_threshold = cfg ? std::max(cfg->big_threshold, 0) : 0;
-    r.given_k_mask = cfg ? cfg->warp_k_mask : 0;
+    const bool whole = cfg && cfg->block_size > 0 && cfg->big_threshold > 0 && cfg->warp_k_mask != 0;
+    r.given_threshold = cfg && !whole ? std::max(cfg->big_threshold, 0) : 0;
+    r.given_k_mask = cfg && !whole ? cfg->warp_k_mask : 0;
     if (cfg) {
         if (cfg->block_size > 0) r.block_size = cfg->block_size;
         if (cfg->big_threshold > 0) r.big_threshold = cfg->big_threshold;
@@ -799,23 +801,32 @@ int hwt_autotune(hwt_ctx *c, const hwt_options *o, const hwt_yield *y, int mode,
                                                    : (mode == HWT_BATCHED_DF64 ? kKMaskFP64 : kKMaskFloatAlt), nullptr)};
     const int n_kmasks = 2;
     double best_ms = 1e300;
-    hwt_config best_cfg = c->tuned[mode];
+    const hwt_config before = c->tuned[mode];
+    hwt_config best_cfg = before, plain;
+    memset(&plain, 0, sizeof(plain));
+    plain.mode = mode;
+    plain.use_graph = 1;
     for (int b : blocks) {
         for (int big : bigs) {
           for (int km = 0; km < n_kmasks; ++km) {
-            hwt_config cfg;
-            memset(&cfg, 0, sizeof(cfg));
-            cfg.mode = mode; cfg.block_size = b; cfg.big_threshold = big; cfg.use_graph = 1;
+            // timed as the context's own configuration, so as the calls that will use it run:
+            // given in the call, the threshold and the K set would be limits, which keep
+            // trees off the polynomial path and uncut
+            hwt_config cfg = plain;
+            cfg.block_size = b;
+            cfg.big_threshold = big;
             cfg.warp_k_mask = kmasks[km];
+            c->tuned[mode] = cfg;
             double t = 1e300;
             for (int k = 0; k < repeats + 1; ++k) {
                 hwt_stats st;
-                r = hwt_price_ex(c, o, y, &cfg, out.data(), &st);
-                if (r == HWT_EUNSUPPORTED) break;
-                if (r) return r;
+                r = hwt_price_ex(c, o, y, &plain, out.data(), &st);
+                if (r) break;
                 if (k > 0) t = std::min(t, st.sizing_ms + st.pricing_ms);
             }
+            c->tuned[mode] = before;
             if (r == HWT_EUNSUPPORTED) continue;
+            if (r) return r;
             // a later (larger) configuration has to win by more than 1%: where the
             // sizes tie (a batch without warp-group trees makes the group size moot)
             // the smaller groups, better for other batches, are kept

@@ -105,7 +105,9 @@ typedef struct hwt_config {
                               double rows, <= 1024 for float rows; 0 = the default).  A value
                               given here is about the whole tree's width: float trees are then
                               not cut to the nodes their paths visit, and wider trees of the
-                              double modes are stepped through instead of summed as polynomials */
+                              double modes are stepped through instead of summed as polynomials.
+                              (A whole record, with block_size, big_threshold and warp_k_mask set
+                              as hwt_get_config and hwt_autotune return them, is no such limit) */
     int32_t use_graph;     /* 1 = replay a captured CUDA graph (default), 0 = direct launches */
     int32_t record_busy;   /* 1 = record per-block busy time for the tail-imbalance stat */
     int32_t warp_k_mask;   /* nodes-per-lane values warp tasks may use: bit q allows the q-th of

@@ -1,6 +1,6 @@
 """The autotuner times the engine that the configured calls run: a tuned or cached
-threshold below the default moves no tree off the paths of an untuned call, and the
-context's own record handed back to a call prices as a call without one."""
+threshold below the default moves no tree off the paths of an untuned call, and a
+whole record handed to a call prices as a context configured with it."""
 import numpy as np
 import pytest
 
@@ -57,14 +57,34 @@ def test_cached_threshold_keeps_the_fast_paths(pkg, pricer, tmp_path, mode_name,
 
 
 @pytest.mark.parametrize("mode_name", ["BATCHED_FP64", "BATCHED_DF64", "BATCHED_MIXED", "BATCHED_FP32"])
-def test_own_record_is_no_limit(pkg, mode_name):
+def test_whole_record_is_no_limit(pkg, mode_name):
     opts, y = _wide(pkg)
     mode = getattr(pkg, mode_name)
     with pkg.Pricer(0) as p:
-        for best in (p.get_config(mode), p.autotune(opts, y, mode, repeats=1)):
+        for record in (lambda: p.get_config(mode), lambda: p.autotune(opts, y, mode, repeats=1)):
+            best = record()
             plain = p.price(opts, y, mode)
             layout = _layout(p)
             again = p.price(opts, y, mode, block_size=best.block_size, big_threshold=best.big_threshold,
                             warp_k_mask=best.warp_k_mask)
             assert _layout(p) == layout
             assert np.array_equal(plain, again)
+
+
+def test_noalloc_float_prices_are_the_uncut_trees(pkg, pricer):
+    """The allocation-free entry point's threshold (512) leaves K = 32 out of its K set; its
+    float trees are cut all the same, with the sums of their uncut layout."""
+    import ctypes
+    torch = pytest.importorskip("torch")
+    opts, y = _wide(pkg)
+    arrays = {"strike": opts.StrikePrices, "bond_maturity": opts.Maturities, "option_maturity": opts.Lengths,
+              "term_unit": opts.TermUnits.view(np.int16), "term_steps": opts.TermStepCounts.view(np.int16),
+              "a": opts.ReversionRates, "sigma": opts.Volatilities, "type": opts.Types}
+    dev = {k: torch.from_numpy(np.ascontiguousarray(v)).cuda() for k, v in arrays.items()}
+    rate, day = torch.from_numpy(y.Prices).cuda(), torch.from_numpy(y.TimeSteps).cuda()
+    out = torch.empty(opts.N, dtype=torch.float64, device="cuda")
+    c_opts, c_yield = pkg._Options(opts.N, *(t.data_ptr() for t in dev.values())), pkg._Yield(y.N, rate.data_ptr(), day.data_ptr())
+    rc = pkg.lib().hwt_price_device_noalloc(ctypes.byref(c_opts), ctypes.byref(c_yield), pkg.BATCHED_FP32, out.data_ptr(), None)
+    assert rc == pkg.HWT_OK
+    uncut = pricer.price(opts, y, pkg.BATCHED_FP32, block_size=64, big_threshold=512)
+    assert np.max(np.abs(out.cpu().numpy() - uncut)) <= 100 * 2.0 ** -46
