@@ -389,7 +389,7 @@ int run_batch(hwt_ctx *c, const DevOptions &dopt, double *dev_out, const RunConf
             if (r) return r;
         }
     }
-    p.s.cta_busy = c->d_busy;
+    p.s.sm_busy = c->d_busy;
     p.tab = c->table;
     poly_params(p, cfg.mode, cfg.given_threshold, cfg.given_k_mask, c->sms, grid);
 

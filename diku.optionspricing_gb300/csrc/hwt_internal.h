@@ -190,7 +190,7 @@ struct Scratch {
     int32_t *bin_start;     // [kKeyBins]
     int32_t *task_start;    // [kKeyBins]
     RunStatus *status;      // [1]
-    unsigned long long *cta_busy; // [max grid] per-CTA busy cycles (tail imbalance)
+    unsigned long long *sm_busy;  // [grid] busy nanoseconds by SM (tail imbalance)
 };
 
 struct EngineParams {

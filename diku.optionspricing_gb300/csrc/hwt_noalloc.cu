@@ -147,7 +147,7 @@ extern "C" int hwt_price_device_noalloc(const hwt_options *dev_opts, const hwt_y
     p.s.bin_start = (int32_t *)(base + kOffBinStart);
     p.s.task_start = (int32_t *)(base + kOffTaskStart);
     p.s.status = (RunStatus *)(base + kOffStatus);
-    p.s.cta_busy = nullptr;
+    p.s.sm_busy = nullptr;
     p.out = dev_out_prices;
     p.max_width = kMaxTreeWidth;
     p.group_threads = mode == HWT_BATCHED_FP64 ? 128 : 64;

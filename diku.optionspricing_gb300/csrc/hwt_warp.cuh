@@ -42,6 +42,18 @@ struct Group {
     int base, nthreads, bar;
 };
 
+// A block's time since t_start, added to its SM's (one thread).  By SM, not by block: the
+// general and the polynomial path's kernels share the SMs, one block of either at a time on
+// each, and block i of one may follow block k of the other.
+__device__ __forceinline__ void add_busy(unsigned long long *sm_busy, unsigned long long t_start)
+{
+    unsigned long long t_end;
+    unsigned sm;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_end));
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+    atomicAdd(&sm_busy[sm % gridDim.x], t_end - t_start);
+}
+
 // The next warp task of a queue (all lanes).
 __device__ __forceinline__ int draw_task(int32_t *counter)
 {

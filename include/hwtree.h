@@ -109,7 +109,7 @@ typedef struct hwt_config {
                               (A whole record, with block_size, big_threshold and warp_k_mask set
                               as hwt_get_config and hwt_autotune return them, is no such limit) */
     int32_t use_graph;     /* 1 = replay a captured CUDA graph (default), 0 = direct launches */
-    int32_t record_busy;   /* 1 = record per-block busy time for the tail-imbalance stat */
+    int32_t record_busy;   /* 1 = record each SM's busy time for the tail-imbalance stat */
     int32_t warp_k_mask;   /* nodes-per-lane values warp tasks may use: bit q allows the q-th of
                               {1, 2, 3, 4, 5, 6, 7, 8, 12, 16, 32}; 12, 16 and 32 apply to float
                               rows only (32: trees of up to 1,024 nodes on one warp, coefficients
@@ -136,8 +136,8 @@ typedef struct hwt_stats {
     int32_t max_width;      /* widest tree in the batch */
     int32_t max_height;     /* tallest tree in the batch */
     int32_t graph_replayed; /* 1 if the kernels ran from a captured graph */
-    double busy_max_ms;     /* per-block busy time: max (record_busy only) */
-    double busy_mean_ms;    /* per-block busy time: mean (record_busy only) */
+    double busy_max_ms;     /* time an SM is busy: max (record_busy only) */
+    double busy_mean_ms;    /* time an SM is busy: mean (record_busy only) */
 } hwt_stats;
 
 typedef struct hwt_ctx hwt_ctx;
