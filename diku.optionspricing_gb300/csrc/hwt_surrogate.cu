@@ -758,16 +758,15 @@ cudaError_t kernel_attributes()
 
 // Tile width: the output width rounded up to 16 (one tile for the 2-wide output
 // layer), at most 128 so that a 256-wide layer spreads over two column tiles.
-constexpr int kFewTiles = 152;
 template <bool TA, bool TB>
-cudaError_t gemm(const GemmArgs &a, int splits, cudaStream_t st)
+cudaError_t gemm(const GemmArgs &a, int splits, int sms, cudaStream_t st)
 {
     if (a.N <= 16) return gemm_bn<TA, TB, 16>(a, splits, st);
     // weight gradients: 128 x 64 tiles while 128 x 128 ones leave SMs without one (batch
     // 8,192: 64 tiles, 19 us; 128 narrower ones 15 us); the others' tiles stay wide (their
     // operand loads, not the tile count, set the time: 17 against 18 us)
     const int tiles = (a.N + 127) / 128 * ((a.M + BM - 1) / BM) * splits;
-    if (a.N <= 64 || (TA && tiles < kFewTiles)) return gemm_bn<TA, TB, 64>(a, splits, st);
+    if (a.N <= 64 || (TA && tiles < sms)) return gemm_bn<TA, TB, 64>(a, splits, st);
     return gemm_bn<TA, TB, 128>(a, splits, st);
 }
 
@@ -812,7 +811,7 @@ int forward_layers(hwt_surrogate *s, int rows)
         g.Cb = to_last ? nullptr : s->d_h[l + 1];
         g.ldcb = kFanOut[l];
         if (to_last) g.epi = EPI_BIAS;
-        SCUDA(s, (gemm<false, false>(g, 1, s->stream)), "forward gemm");
+        SCUDA(s, (gemm<false, false>(g, 1, s->sms, s->stream)), "forward gemm");
     }
     layer4_kernel<<<(2 * rows + 63) / 64, 64, 0, s->stream>>>(s->d_z[kLayers - 2], s->d_w + s->w_off[kLayers - 1],
                                                              s->d_w + s->b_off[kLayers - 1], rows, s->d_z[kLayers - 1]);
@@ -889,7 +888,7 @@ int backward(hwt_surrogate *s, int rows, float lam, bool zero_loss)
         gw.ldc = out;
         gw.k_chunk = kc;
         const int zs = (rows + kc - 1) / kc;  // every slice holds at least one K block
-        SCUDA(s, (gemm<true, true>(gw, zs, s->stream)), "dW gemm");
+        SCUDA(s, (gemm<true, true>(gw, zs, s->sms, s->stream)), "dW gemm");
         SCUDA(s, reduce(zs, in * out, s->d_g + s->w_off[l]), "dW sum");
         // db_l = column sums of dZ_l (fp32 copy in d_dzf)
         dim3 cg((out + 255) / 256, nslice);
@@ -903,7 +902,7 @@ int backward(hwt_surrogate *s, int rows, float lam, bool zero_loss)
         gd.ldc = in;
         gd.Cb = dz_next;
         gd.ldcb = in;
-        SCUDA(s, (gemm<false, false>(gd, 1, s->stream)), "dX gemm");
+        SCUDA(s, (gemm<false, false>(gd, 1, s->sms, s->stream)), "dX gemm");
         std::swap(dz, dz_next);
     }
     // layer 0 in fp32: dW0 = X^T dZ0, db0 = column sums of dZ0
