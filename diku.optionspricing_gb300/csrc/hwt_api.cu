@@ -306,6 +306,14 @@ __global__ void fetch_options_kernel(DevOptions src, DevOptions dst)
     const_cast<int8_t *>(dst.type)[i] = ty;
 }
 
+// Leaves a host call whose launches failed part-way: not before the kernels that are under
+// way have read the caller's arrays, which the caller may free on return.
+int abandon(hwt_ctx *c, int r)
+{
+    cudaStreamSynchronize(c->stream);
+    return r;
+}
+
 std::string bad_option_message(const RunStatus &st)
 {
     const unsigned long long fb = st.first_bad;
@@ -648,7 +656,7 @@ int hwt_price_ex(hwt_ctx *c, const hwt_options *o, const hwt_yield *y, const hwt
         // from the pricing kernel, 8 scattered bytes per option, they cost the
         // kernel ~5%).
         if (stats) HWT_CUDA(c, cudaEventRecord(c->ev[0], c->stream), "event");
-        if ((r = run_batch(c, host, c->d_out, cfg, stats, &launches, &graph_used))) return r;
+        if ((r = run_batch(c, host, c->d_out, cfg, stats, &launches, &graph_used))) return abandon(c, r);
         HWT_CUDA(c, cudaMemcpyAsync(out, c->d_out, 8 * n, cudaMemcpyDeviceToHost, c->stream), "prices D2H");
         r = finish(c, cfg, stats, launches, graph_used, grid, 45 * n, 8 * n);
         if (stats) timing_fill(c, stats, c->ev[0]);
@@ -689,7 +697,7 @@ int hwt_price_ex(hwt_ctx *c, const hwt_options *o, const hwt_yield *y, const hwt
                                         c->stream), "options H2D");
         }
     }
-    if ((r = run_batch(c, dopt, c->d_out, cfg, stats, &launches, &graph_used))) return r;
+    if ((r = run_batch(c, dopt, c->d_out, cfg, stats, &launches, &graph_used))) return abandon(c, r);
     launches += launches_before;
     double *dst = out_pinned ? out : c->h_out;
     HWT_CUDA(c, cudaMemcpyAsync(dst, c->d_out, 8 * n, cudaMemcpyDeviceToHost, c->stream), "prices D2H");
