@@ -54,6 +54,31 @@ WORKLOAD_NAMES = ["uniform_1k", "uneven_30k", "skewed_100k", "0_uniform", "1_ran
                   "3_randconstwidth", "4_skewed", "5_skewedconstheight", "6_skewedconstwidth"]
 
 
+def kept_nodes(pkg, opts, shp) -> int:
+    """Active nodes of one pass over float trees as the engine cuts them: to the nodes that
+    paths of sqrt(8.25^2 + z^2) standard deviations visit, z the option's own distance out
+    of the money (the rule of the sizing pass, csrc/hwt_batched.cu, in numpy)."""
+    wl = pkg.workloads
+    rates, days = wl.yield_curve()
+    n, jmax, m = (shp[k].astype(np.int64) for k in ("height", "jmax", "maturity_step"))
+    unit = opts.TermUnits.astype(np.int64)
+    dt = -(-365 // unit) / opts.TermStepCounts.astype(np.float64)
+    adt = opts.ReversionRates * dt
+    drdt = opts.Volatilities * np.sqrt(3.0 * -np.expm1(-2.0 * adt) / (2.0 * opts.ReversionRates)) * dt
+    pays = (m >= 1) & (m < n)
+    mm = np.where(pays, m, 1)
+    away = np.log(opts.StrikePrices / wl.forward_bond_price(mm * dt, n * dt, rates, days))
+    otm = np.maximum(np.where(opts.Types == 1, -away, away), 0.0)
+    slope = drdt * np.expm1(-adt * (n - mm)) / np.expm1(-adt)
+    var = -np.expm1(-2.0 * adt * mm) / (6.0 * adt)
+    nowhere = otm > slope * (np.minimum(mm, jmax) + 2.0 + 2.0 * slope * var)
+    z = np.where(pays & ~nowhere, otm / (slope * np.sqrt(var)), 0.0)
+    back = -np.expm1(-0.75 * adt * n)
+    reach = (np.sqrt((8.25 ** 2 + z * z) * -np.expm1(-2.0 * adt * n) / (6.0 * adt)) +
+             drdt / (3.0 * adt * adt) * back * back + 2.0)
+    return int(np.sum(pkg.active_nodes(n, np.minimum(jmax, reach.astype(np.int64) + 1))))
+
+
 def dist_env():
     rank = int(os.environ.get("RANK", "0"))
     world = int(os.environ.get("WORLD_SIZE", "1"))
@@ -291,7 +316,7 @@ def config_runs(pkg, orc, pricer, y, reps: int) -> dict:
     got, ms, st = run(sk, pkg.PLAIN_FP64)
     entry["plain_fp64_one_block_per_option"] = {"device_ms": ms, "options_per_s": sk.N / (ms * 1e-3),
                                                 **errors(got, ref)}
-    entry["note"] = ("tail = busiest pricing block / mean block busy time - 1; the reference's cuda-multi rejects "
+    entry["note"] = ("tail = busiest SM / mean SM busy time - 1; the reference's cuda-multi rejects "
                      "trees wider than 1,024 nodes (cuda-multi/Kernel.cuh:395-400), so it cannot price this batch")
     out["skewed_100k"] = entry
     return out
@@ -448,7 +473,6 @@ def run_ours(args, rank, world, local):
     n = opts.N
     shp = pkg.shape(opts)
     nodes = int(np.sum(pkg.active_nodes(shp["height"], shp["jmax"])))
-    flop_per_batch = FLOP_PER_NODE * nodes
 
     pricer = pkg.Pricer(local)
     if args.network_rows:
@@ -671,7 +695,10 @@ def run_ours(args, rank, world, local):
     peaks = pricer.measure_peaks()
     measured = load_json(os.path.join(ROOT, "MEASURED_PEAKS.json")) or {}
     fp32_peak = peaks[1]
-    achieved = flop_per_batch / (pricing_ms * 1e-3) / 1e12
+    # float rows: the nodes of the cut trees; the double modes sum their rows as polynomials,
+    # for which no count of nodes stands (their pipes' use is in the profiles)
+    work_nodes = {"mixed": kept_nodes(pkg, opts, shp), "fp32": kept_nodes(pkg, opts, shp), "plain": nodes}.get(args.mode)
+    achieved = None if work_nodes is None else FLOP_PER_NODE * work_nodes / (pricing_ms * 1e-3) / 1e12
     prof = load_json(os.path.join(ROOT, "profiles", f"pricing_{args.workload}_{args.mode}.json")) or {}
     traffic = prof.get("dram_bytes_per_launch")
     bound = {"mixed": "fp32", "fp32": "fp32", "fp64": "fp64", "df64": "fp32", "plain": "fp64"}[args.mode]
@@ -705,9 +732,10 @@ def run_ours(args, rank, world, local):
                     int(sum(t.numel() * t.element_size() for t in sub_host.values())) + 8 * len(mine),
                     "d2h_bytes_per_step": 8 * n if parts is None else 8 * len(mine) + 8 * n},
             "roofline": {"bound": bound, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                         "frac": achieved / peak, "traffic": traffic,
-                         "work": f"{FLOP_PER_NODE} FLOP x {nodes} active nodes per launch; peak = FMA microbenchmark "
-                                 f"on this GPU (MEASURED_PEAKS.json has no FP32/FP64 entries; its HBM figure is "
+                         "frac": None if achieved is None else achieved / peak, "traffic": traffic,
+                         "work": (f"{FLOP_PER_NODE} FLOP x {work_nodes} nodes per launch, of {nodes} active ones; "
+                                  if work_nodes is not None else "rows summed as polynomials: no fixed count; ") +
+                                 f"peak = FMA microbenchmark on this GPU (MEASURED_PEAKS.json has no FP32/FP64 entries; its HBM figure is "
                                  f"{measured.get('hbm_gbs')} GB/s)",
                          "kernel_ms": pricing_ms},
             "peaks_measured": {"fp64_tflops": peaks[0], "fp32_tflops": peaks[1]},
