@@ -802,7 +802,7 @@ int hwt_autotune(hwt_ctx *c, const hwt_options *o, const hwt_yield *y, int mode,
     if (o->n == 0) return fail(c, HWT_EINVAL, "autotune needs a non-empty batch");
     std::vector<double> out(o->n);
     const int blocks[] = {64, 128, 256, 512};
-    const int bigs[] = {128, 256, 384, 512, 1024};
+    const int bigs[] = {1024, 512, 384, 256, 128};
     // the mode's default K set and a denser one (better fit, larger code footprint)
     const int kmasks[] = {resolve_k_mask(mode, 0, nullptr),
                           resolve_k_mask(mode, mode == HWT_BATCHED_FP64 ? kKMaskFP64Alt
@@ -816,6 +816,7 @@ int hwt_autotune(hwt_ctx *c, const hwt_options *o, const hwt_yield *y, int mode,
     plain.use_graph = 1;
     for (int b : blocks) {
         for (int big : bigs) {
+          if (wide_rows(mode) && big > kDefaultBig) continue;  // (their warp tasks end there)
           for (int km = 0; km < n_kmasks; ++km) {
             // timed as the context's own configuration, so as the calls that will use it run:
             // given in the call, the threshold and the K set would be limits, which keep
@@ -835,9 +836,11 @@ int hwt_autotune(hwt_ctx *c, const hwt_options *o, const hwt_yield *y, int mode,
             c->tuned[mode] = before;
             if (r == HWT_EUNSUPPORTED) continue;
             if (r) return r;
-            // a later (larger) configuration has to win by more than 1%: where the
-            // sizes tie (a batch without warp-group trees makes the group size moot)
-            // the smaller groups, better for other batches, are kept
+            // a later configuration has to win by more than 1%: where the sizes tie (a
+            // batch without warp-group trees makes the group size moot, one of narrow
+            // trees the threshold) the smaller groups and wider warp tasks, better for
+            // other batches, are kept (the skewed batch priced with what ties on the
+            // uneven one: 0.9 ms mixed, 2.3 ms at the smallest threshold that does)
             if (t < 0.99 * best_ms || best_ms == 1e300) { best_ms = t; best_cfg = cfg; }
           }
         }
