@@ -68,6 +68,7 @@ constexpr int kKMaskFP64Alt = 0xAF;   // autotuner's alternative: 1, 2, 3, 4, 6,
 constexpr int kKMaskFloat = 0x68B;    // default K set of float rows: 1, 2, 4, 8, 16, 32
 constexpr int kKMaskFloatAlt = 0x7AF; // autotuner's alternative: 1, 2, 3, 4, 6, 8, 12, 16, 32
 constexpr int kKMaskAll = 0x7FF;      // what a caller may ask for
+constexpr int kKMaskShort = 0x0F;     // of a mode's K set: 1 .. 4
 constexpr int kKMaskCut = 0x920;      // added for cut trees: 6, 10, 12
 constexpr int kNumL = 6;                       // L = 1, 2, 4, 8, 16, 32
 constexpr int kClsMask = 127;                  // class word: K and L indices in bits 0-6,

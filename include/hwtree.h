@@ -220,7 +220,8 @@ int64_t hwt_active_nodes(int32_t height, int32_t jmax);
 /* How the batched engine lays out an uncut tree `width` nodes wide, stepped through, for `mode` (a batched
  * mode) with this K mask and widest-warp-task threshold (0 = the defaults, as a
  * context without tuning uses them; hwt_price_device_noalloc uses threshold 512
- * for the float modes and 256 for FP64): *K nodes per lane on *L lanes of a warp task,
+ * for the float modes and 256 for FP64; trees that the double modes step through only for
+ * being far out of the money take 4 nodes a lane at most): *K nodes per lane on *L lanes of a warp task,
  * or *K = *L = 0 when the tree goes to a warp group.  Host only, no GPU.
  * HWT_EINVAL for a non-batched mode or a width outside 1..4096. */
 int hwt_warp_layout(int mode, int32_t width, int32_t warp_k_mask, int32_t big_threshold, int32_t *K,
