@@ -109,7 +109,7 @@ constexpr int kPolyGroupK = 0xAB;       // 1, 2, 4, 6, 8
 constexpr int kPolyKFP64 = 0xFF;        // 1 .. 8
 constexpr int kPolyKDF64 = 0xAA;        // 2, 4, 6, 8 (pairs)
 // threads of a block: double mode's fixed-point rows need 168 registers (at 128 their
-// step loops spilled), double-float rows do with 128
+// step loops spilled 1.3 KB); double-float rows run at 128, with some 350 bytes of spills
 constexpr int kPolyThreadsFP64 = 384;
 constexpr int kPolyThreadsDF64 = 512;
 constexpr int kPolyMaxJ = 128 * 8 / 2 - 1;
